@@ -49,7 +49,7 @@ enum { VG_PROBLEM_SINCOS = 1, VG_PROBLEM_SINSIN = 2, VG_PROBLEM_ANNULUS = 3 };
 enum { VG_BC_FLUX = 0, VG_BC_PRESSURE = 1 };
 enum { VG_FP64 = 0, VG_FP32 = 1 };
 /* solve modes: FP64 throughout, or FP32 inner solves under FP64 iterative refinement (degree 0 on small
- * meshes: FP64 inner solves, which are the faster ones there) */
+ * meshes of a problem with sources: FP64 inner solves, which are the faster ones there) */
 enum { VG_SOLVE_FP64 = 0, VG_SOLVE_MIXED = 1 };
 
 /* The reference reader's StraightMeshData (vem/CurvedVEM_Darcy_gpu/mesh/straight_mesh.h:20-49),
@@ -193,7 +193,9 @@ void vg_default_solve_opts(vg_solve_opts* opts);
 /* Solve A x = b to ||b - A x|| / ||b|| <= opts->tol (device pointers). Replaces Krylov::solve
  * (vem/CurvedVEM_Darcy_gpu/src/krylov.cu:73-175); PETSc FGMRES is replaced by conjugate
  * gradients on the edge pressures (fluxes and pressures eliminated cell by cell) with a multigrid
- * preconditioner, the FP64 true-residual acceptance is kept. */
+ * preconditioner, the FP64 true-residual acceptance is kept. Degree 0, pressure condition, VG_PROBLEM_ANNULUS (no
+ * sources), up to 32,768 cells: MINRES on the saddle-point form, so that the divergence vg_errors reports there, which is
+ * the residual of the solve, stays the figure on record. */
 int vg_solve(vg_handle* h, const double* b, double* x, const vg_solve_opts* opts, vg_solve_info* info);
 
 /* Same with host buffers: copies b in and x out inside the call (the end-to-end path). */

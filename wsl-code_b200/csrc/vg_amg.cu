@@ -854,6 +854,40 @@ __global__ void __launch_bounds__(256) k_gj_step(const double* __restrict__ a, d
     for (int i = 0; i < GJ_B; ++i) Dn[i * GJ_B + t] = v[i];
 }
 
+// One pivot k a launch, in place, with column k and row k saved before the step (ncol, nrow: the next step's):
+//   a_kk <- 1/p, a_kj <- a_kj/p, a_ik <- -a_ik/p, a_ij <- a_ij - a_ik a_kj / p   (p = a_kk)
+// It reads and writes the whole matrix n times (a mesh of 2,400 cells, whose graph is its coarsest level, is created and
+// built in 84 ms, by panels in 14). Its last bits decide the figures of the meshes that MINRES solves.
+__global__ void k_gj_pivot(double* a, int n, int k, const double* col, const double* row, unsigned long long* bad,
+                           double* ncol, double* nrow) {
+    const long long t = blockIdx.x * (long long)TPB + threadIdx.x;
+    if (t >= (long long)n * n) return;
+    const int i = int(t / n), j = int(t % n);
+    const double p = row[k];
+    if (!(p > 0.0)) {  // not positive definite: reported, the result is not used
+        if (t == 0) *bad = 1ull;
+        return;
+    }
+    double v;
+    if (i == k && j == k)
+        v = 1.0 / p;
+    else if (i == k)
+        v = row[j] / p;
+    else if (j == k)
+        v = -col[i] / p;
+    else
+        v = a[t] - col[i] * row[j] / p;
+    a[t] = v;
+    if (j == k + 1) ncol[i] = v;
+    if (i == k + 1) nrow[j] = v;
+}
+__global__ void k_gj_save(const double* a, int n, double* col, double* row) {  // column and row 0
+    const int t = blockIdx.x * TPB + threadIdx.x;
+    if (t >= n) return;
+    col[t] = a[(long long)t * n];
+    row[t] = a[t];
+}
+
 // symmetric part in FP64 and FP32 (the exact inverse is symmetric)
 __global__ void k_gj_sym(const double* a, int n, double* o64, float* o32) {
     long long t = blockIdx.x * (long long)TPB + threadIdx.x;
@@ -996,7 +1030,7 @@ inline int blocks(int n) { return (n + TPB - 1) / TPB; }
 
 }  // namespace
 
-void Amg::dense_inverse(const int* ptr, const int* col, const double* val, int n) {
+void Amg::dense_inverse(const int* ptr, const int* col, const double* val, int n, bool pivotwise) {
     const size_t nn = size_t(n) * n;
     const int panels = (n + GJ_B - 1) / GJ_B, tiles = (n + GJ_T - 1) / GJ_T;
     gj_work_.resize(nn);
@@ -1005,16 +1039,29 @@ void Amg::dense_inverse(const int* ptr, const int* col, const double* val, int n
     dinvc64_.resize(nn);
     dinvc32_.resize(nn);
     gj_bad_.zero();
-    // the panels go back and forth between the two copies and end in gj_work_
-    double* cur = panels % 2 ? dinvc64_.data() : gj_work_.data();
-    double* nxt = panels % 2 ? gj_work_.data() : dinvc64_.data();
+    // the panels go back and forth between the two copies and end in gj_work_; the pivots stay there
+    const bool odd = panels % 2 && !pivotwise;
+    double* cur = odd ? dinvc64_.data() : gj_work_.data();
+    double* nxt = odd ? gj_work_.data() : dinvc64_.data();
     k_csr_dense<<<std::min(2 * 148, (n + TPB / 32 - 1) / (TPB / 32)), TPB>>>(ptr, col, val, n, constant_kernel_, cur);
-    k_gj_first<<<1, 32>>>(cur, n, gj_d_.data(), gj_bad_.data());
-    for (int i = 0; i < panels; ++i) {
-        double* D = gj_d_.data() + i % 2 * (GJ_B * GJ_B);
-        double* Dn = gj_d_.data() + (i + 1) % 2 * (GJ_B * GJ_B);
-        k_gj_step<<<dim3(tiles, tiles), 256>>>(cur, nxt, n, i * GJ_B, D, Dn, gj_bad_.data());
-        std::swap(cur, nxt);
+    if (pivotwise) {
+        DevBuf<double> edge(4 * size_t(n));
+        double *c0 = edge.data(), *r0 = c0 + n, *c1 = r0 + n, *r1 = c1 + n;
+        k_gj_save<<<blocks(n), TPB>>>(cur, n, c0, r0);
+        for (int k = 0; k < n; ++k) {
+            k_gj_pivot<<<int((nn + TPB - 1) / TPB), TPB>>>(cur, n, k, c0, r0, gj_bad_.data(), c1, r1);
+            std::swap(c0, c1);
+            std::swap(r0, r1);
+        }
+        VG_CUDA(cudaDeviceSynchronize());  // edge goes
+    } else {
+        k_gj_first<<<1, 32>>>(cur, n, gj_d_.data(), gj_bad_.data());
+        for (int i = 0; i < panels; ++i) {
+            double* D = gj_d_.data() + i % 2 * (GJ_B * GJ_B);
+            double* Dn = gj_d_.data() + (i + 1) % 2 * (GJ_B * GJ_B);
+            k_gj_step<<<dim3(tiles, tiles), 256>>>(cur, nxt, n, i * GJ_B, D, Dn, gj_bad_.data());
+            std::swap(cur, nxt);
+        }
     }
     k_gj_sym<<<int((nn + TPB - 1) / TPB), TPB>>>(cur, n, dinvc64_.data(), dinvc32_.data());
     VG_CUDA(cudaGetLastError());
@@ -1098,10 +1145,12 @@ long long Amg::nnz() const {
     return t;
 }
 
-void Amg::setup(const HostCsr& S0, int* err, const std::vector<int>* fine_order, bool constant_kernel) {
+void Amg::setup(const HostCsr& S0, int* err, const std::vector<int>* fine_order, bool constant_kernel,
+                bool saddle) {
     PhaseTimer pt;
     err_ = err;
     constant_kernel_ = constant_kernel;
+    saddle_ = saddle;
     levels_.clear();
     release_streams();
     HostCsr A = S0;
@@ -1217,7 +1266,7 @@ void Amg::setup(const HostCsr& S0, int* err, const std::vector<int>* fine_order,
             } else {
                 const double rho = rho_dinv_a(A, dinv_own);
                 L.omega = 4.0 / (3.0 * rho);
-                L.smooth = SMOOTH_WEIGHT / rho;
+                L.smooth = saddle ? L.omega : SMOOTH_WEIGHT / rho;
                 P = smoothed_prolongator(A, agg, nagg, dinv_own, L.omega);
                 L.agg.resize(A.n);
                 for (int i = 0; i < A.n; ++i) L.agg[fine ? (*fine_order)[i] : i] = agg[i];
@@ -1320,7 +1369,7 @@ void Amg::setup(const HostCsr& S0, int* err, const std::vector<int>* fine_order,
         if (pt.on) VG_CUDA(cudaDeviceSynchronize());
         pt.mark("multigrid uploads");
         const Level& C = levels_.back();
-        dense_inverse(C.dpa_ptr.data(), C.dpa_col.data(), v.data(), C.n);
+        dense_inverse(C.dpa_ptr.data(), C.dpa_col.data(), v.data(), C.n, saddle_);
         pt.mark("coarsest dense inverse");
     }
     prepare_csr_kernels(csr_slots_);

@@ -93,8 +93,11 @@ public:
     // after S has been coarsened in its own order; err: the device address of
     // the owner's error word; constant_kernel: S has the constants as its kernel (so
     // has every coarse matrix, whose aggregates' prolongator keeps them), and the coarsest one is inverted
-    // with the mean of its diagonal as the constants' eigenvalue
-    void setup(const HostCsr& S, int* err, const std::vector<int>* fine_order = nullptr, bool constant_kernel = false);
+    // with the mean of its diagonal as the constants' eigenvalue; saddle: the hierarchy of MINRES (vg_minres.cu),
+    // whose figures are to the bit those of the prolongator's weight in the smoother and of a coarsest inverse
+    // formed pivot by pivot
+    void setup(const HostCsr& S, int* err, const std::vector<int>* fine_order = nullptr, bool constant_kernel = false,
+               bool saddle = false);
     bool ready() const { return !levels_.empty(); }
     int levels() const { return int(levels_.size()); }
     long long nnz() const;
@@ -163,7 +166,8 @@ private:
     };
     template <typename T>
     void cycle(int l, const T* b, T* z, cudaStream_t s);
-    void dense_inverse(const int* ptr, const int* col, const double* val, int n);  // CSR -> dinvc64_ / dinvc32_
+    // CSR -> dinvc64_ / dinvc32_, by panels or pivot by pivot
+    void dense_inverse(const int* ptr, const int* col, const double* val, int n, bool pivotwise = false);
     template <typename T>
     DevSell<T> view(const Level& L) const;
     template <typename T>
@@ -171,7 +175,7 @@ private:
 
     std::vector<Level> levels_;
     int ncoarse_ = 0;
-    bool constant_kernel_ = false;
+    bool constant_kernel_ = false, saddle_ = false;
     int* err_ = nullptr;  // the owner's error word: set when a cycle kernel gave up on a copy (never in a correct run)
     int csr_slots_[2] = {1, 1};  // resident CTAs of the CSR kernels on this hierarchy's device (FP32, FP64)
     DevBuf<double> dinvc64_;  // dense inverse of the coarsest matrix

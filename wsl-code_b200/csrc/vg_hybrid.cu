@@ -567,10 +567,7 @@ void Solver::prepare_hybrid() {
     pt.mark("edge system: values");
     if (use_amg) {
         d_lap_.resize(size_t(amg_.level0_nnz()));
-        k_laplacian<<<hblocks(m.nc), HT>>>(amg_.level0_ptr(), amg_.level0_col(), m.nc, d_rank_slot_.data(),
-                                           d_pieces_.data(), d_emap_.data(), d_ecell_.data(), d_econd_.data(),
-                                           d_lap_.data());
-        VG_CUDA(cudaGetLastError());
+        laplacian_values(amg_, d_econd_.data(), d_lap_.data());
         amg_.refresh(d_lap_.data());
         pt.mark("multigrid refresh");
     } else {
@@ -591,7 +588,24 @@ std::vector<int> Solver::rank_order() const {
 // multigrid of the cells' graph Laplacian (see the head of the file); without it (a hierarchy that does
 // not coarsen) the diagonal alone preconditions
 void Solver::build_amg() {
-    std::vector<double> cond = d_econd_.download();
+    const std::vector<double> own = d_econd_.download();
+    std::vector<double> cond(m.ne);
+    for (int e = 0; e < m.ne; ++e) cond[e] = own[edge_order_[e]];
+    const HostCsr S = cell_graph(cond);
+    const std::vector<int> order = rank_order();
+    use_amg = false;
+    amg_levels = 0;
+    try {
+        amg_.setup(S, d_errp_, &order, bc == VG_BC_FLUX);
+    } catch (const Error& e) {
+        if (e.code == VG_ENOMEM || e.code == VG_ECUDA) throw;
+        return;
+    }
+    amg_levels = amg_.levels();
+    use_amg = true;
+}
+
+HostCsr Solver::cell_graph(const std::vector<double>& cond) const {
     std::vector<int> ec(2 * size_t(m.ne), -1);
     for (int c = 0; c < m.nc; ++c)
         for (int j = m.cptr[c]; j < m.cptr[c + 1]; ++j) {
@@ -607,7 +621,7 @@ void Solver::build_amg() {
         double diag = 0;
         for (int j = m.cptr[c]; j < m.cptr[c + 1]; ++j) {
             const int e = m.gedges[j];
-            const double d = cond[edge_order_[e]];
+            const double d = cond[e];
             diag += d;
             const int o = ec[2 * e] == c ? ec[2 * e + 1] : ec[2 * e];
             if (o >= 0) row.push_back({o, -d});
@@ -624,17 +638,13 @@ void Solver::build_amg() {
         }
         S.ptr[c + 1] = int(S.col.size());
     }
-    const std::vector<int> order = rank_order();
-    use_amg = false;
-    amg_levels = 0;
-    try {
-        amg_.setup(S, d_errp_, &order, bc == VG_BC_FLUX);
-    } catch (const Error& e) {
-        if (e.code == VG_ENOMEM || e.code == VG_ECUDA) throw;
-        return;
-    }
-    amg_levels = amg_.levels();
-    use_amg = true;
+    return S;
+}
+
+void Solver::laplacian_values(const Amg& amg, const double* cond, double* val) {
+    k_laplacian<<<hblocks(m.nc), HT>>>(amg.level0_ptr(), amg.level0_col(), m.nc, d_rank_slot_.data(), d_pieces_.data(),
+                                       d_emap_.data(), d_ecell_.data(), cond, val);
+    VG_CUDA(cudaGetLastError());
 }
 
 // ---- solve ----------------------------------------------------------------------------------------
@@ -869,7 +879,7 @@ void Solver::solve(const double* b, double* x, const vg_solve_opts& o, vg_solve_
     if (!(o.tol > 0) || o.maxit < 1 || o.check_every < 0 || (o.mode == VG_SOLVE_MIXED && !(o.inner_tol > 0 && o.inner_tol < 1)))
         throw Error(VG_EINVAL, "invalid solve options");
     info = vg_solve_info{};
-    if (!hybrid_ready_) prepare_hybrid();
+    if (!hybrid_ready_ && !minres_.ready) prepare_hybrid();
     (void)s;
     s = stream_;
     // order after the caller's work on the legacy default stream
@@ -909,6 +919,16 @@ void Solver::solve(const double* b, double* x, const vg_solve_opts& o, vg_solve_
         rel = read();
     }
     int total = 0, outer = 0;
+    if (minres_.ready) {
+        if (!guess) rel = read();  // |b|
+        const double nb = std::sqrt(out.red[1]);
+        minres_solve(x, r.data(), nb > 0 ? nb : 1.0, o,
+                     [&] {
+                         true_residual();
+                         return read();
+                     },
+                     rel, total, outer, s);
+    }
     // A correction aims at a tenth of the tolerance (the reference's KSP factor, krylov.cu:142), in the
     // preconditioned norm and in the flux jumps, which are what the residual's rows will see of the error; the true FP64
     // residual then decides (krylov.cu:136-170) and a further correction follows while they gain. A loop's gain in its
@@ -919,10 +939,10 @@ void Solver::solve(const double* b, double* x, const vg_solve_opts& o, vg_solve_
     // us: 100 cells 328 -> 263, 1,000 386 -> 305, 8,000 549 -> 452, 45,000 923 -> 806). From degree 1 on the FP64
     // blocks cost what they spare (10,000 cells 981 against 1,052, degree 2 40,000 cells 14,851 against 16,482).
     const bool fp64 = o.mode == VG_SOLVE_FP64 || (k == 0 && o.check_every <= 0 && takes_one_launch<double>());
-    const int steps = o.mode == VG_SOLVE_FP64 ? 12 : o.max_outer;
+    const int steps = minres_.ready ? 0 : o.mode == VG_SOLVE_FP64 ? 12 : o.max_outer;
     double ratio = 1.0;
     int idle = 0;
-    for (outer = 0; outer < steps && rel > o.tol && total < o.maxit; ++outer) {
+    for (; outer < steps && rel > o.tol && total < o.maxit; ++outer) {
         const double want = 0.1 * o.tol / (rel * ratio), before = rel;
         CgStop stop;
         stop.raw = 0.1 * o.tol;

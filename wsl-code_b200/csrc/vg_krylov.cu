@@ -299,6 +299,201 @@ __global__ void __launch_bounds__(VEC_THREADS) k_cg_direction(CgVecs<T> v, const
         });
 }
 
+// ---- MINRES (Paige-Saunders, unnormalised Lanczos vectors, symmetric positive definite preconditioner) ----
+__device__ void minres_start(MinresScalars* sc, int* flags, double g2, double tol) {
+    const double g = sqrt(fmax(g2, 0.0));
+    sc->gam = g;
+    sc->gam_prev = 1.0;
+    sc->c_prev = 1.0;
+    sc->c = 1.0;
+    sc->s_prev = 0.0;
+    sc->s = 0.0;
+    sc->eta = g;
+    sc->eta0 = g;
+    sc->tol = tol;
+    flags[0] = (g > 0 && isfinite(g)) ? 0 : 1;
+    flags[1] = 0;
+    flags[2] = 0;
+}
+
+// Givens rotation and residual estimate once gamma_{j+1}^2 is known
+__device__ void minres_scalars(MinresScalars* sc, int* flags, double gn2) {
+    const double g = sc->gam, dl = sc->delta / (g * g);
+    const double gn = sqrt(fmax(gn2, 0.0));
+    const double c = sc->c, cp = sc->c_prev, s = sc->s, sp = sc->s_prev, eta = sc->eta;
+    const double a0 = c * dl - cp * s * g;
+    const double a1 = sqrt(a0 * a0 + gn * gn);
+    const double a2 = s * dl + cp * c * g;
+    const double a3 = sp * g;
+    const bool ok = a1 > 0 && isfinite(a1);
+    const double cn = ok ? a0 / a1 : 1.0, sn = ok ? gn / a1 : 0.0;
+    sc->a1 = ok ? a1 : 1.0;
+    sc->a2 = a2;
+    sc->a3 = a3;
+    sc->zscale = 1.0 / g;
+    sc->xcoef = ok ? cn * eta : 0.0;
+    sc->eta = -sn * eta;
+    sc->c_prev = c;
+    sc->c = cn;
+    sc->s_prev = s;
+    sc->s = sn;
+    sc->gam_prev = g;
+    sc->gam = gn;
+    flags[1] = ok ? 1 : 0;
+    flags[2] += 1;
+    if (!ok || !(gn > 0) || fabs(sc->eta) <= sc->tol * sc->eta0) flags[0] = 1;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(VEC_THREADS) k_minres_init(const T* r, MinresVecs<T> v, MinresScalars* sc,
+                                                             double* partials, unsigned* counter) {
+    double acc[1] = {0};
+    auto one = [&](long long i) {
+        const T ri = r[i];
+        v.v_cur[i] = ri;
+        v.v_old[i] = v.w_cur[i] = v.w_old[i] = v.y[i] = T(0);
+        if (i < v.nf) {
+            const T zi = v.dinv[i] * ri;
+            v.z_cur[i] = zi;
+            acc[0] += double(zi) * double(ri);
+        }
+    };
+    for_range(
+        0, v.n,
+        [&](long long i) {
+            if (i < v.nf && i + 3 >= v.nf) {  // the four entries at the end of the flux rows
+                for (int j = 0; j < 4; ++j) one(i + j);
+                return;
+            }
+            T r4[4], z0[4] = {T(0), T(0), T(0), T(0)};
+            ld4(r + i, r4);
+            st4(v.v_cur + i, r4);
+            st4(v.v_old + i, z0);
+            st4(v.w_cur + i, z0);
+            st4(v.w_old + i, z0);
+            st4(v.y + i, z0);
+            if (i >= v.nf) return;
+            T d4[4], zi[4];
+            ld4(v.dinv + i, d4);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                zi[j] = d4[j] * r4[j];
+                acc[0] += double(zi[j]) * double(r4[j]);
+            }
+            st4(v.z_cur + i, zi);
+        },
+        one);
+    grid_reduce<1>(acc, partials, counter, [&](double* tot) { sc->dot = tot[0]; });
+}
+
+template <bool FLUX, typename T>
+__global__ void __launch_bounds__(VEC_THREADS) k_minres_update(MinresVecs<T> v, MinresScalars* sc, int* flags,
+                                                               double* partials, unsigned* counter) {
+    // the first V-cycle kernel after this one (launched with programmatic dependent launch) may
+    // start now and copy its matrix rows while the update runs; it waits for the update's results
+    pdl_trigger();
+    if (flags[0]) {
+        if (FLUX && blockIdx.x == 0 && threadIdx.x == 0) flags[1] = 0;
+        return;
+    }
+    const double g = sc->gam, gp = sc->gam_prev, dl = sc->delta / (g * g);
+    const T f1 = T(1.0 / g), f2 = T(dl / g), f3 = T(g / gp);
+    double acc[1] = {0};
+    for_range(
+        FLUX ? 0 : v.nf, FLUX ? v.nf : v.n,
+        [&](long long i) {
+            T y4[4], vc[4], vo[4], vn[4], z0[4] = {T(0), T(0), T(0), T(0)};
+            ld4(v.y + i, y4);
+            ld4(v.v_cur + i, vc);
+            ld4(v.v_old + i, vo);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) vn[j] = y4[j] * f1 - f2 * vc[j] - f3 * vo[j];
+            st4(v.v_old + i, vn);
+            st4(v.y + i, z0);
+            if (!FLUX) return;
+            T d4[4], zn[4];
+            ld4(v.dinv + i, d4);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                zn[j] = d4[j] * vn[j];
+                acc[0] += double(zn[j]) * double(vn[j]);
+            }
+            st4(v.z_new + i, zn);
+        },
+        [&](long long i) {
+            const T vn = v.y[i] * f1 - f2 * v.v_cur[i] - f3 * v.v_old[i];
+            v.v_old[i] = vn;
+            v.y[i] = T(0);
+            if (!FLUX) return;
+            const T zn = v.dinv[i] * vn;
+            v.z_new[i] = zn;
+            acc[0] += double(zn) * double(vn);
+        });
+    if (FLUX) grid_reduce<1>(acc, partials, counter, [&](double* tot) { sc->dot = tot[0]; });
+}
+
+template <typename T>
+__global__ void __launch_bounds__(VEC_THREADS) k_minres_finish(const T* z, const T* vv, long long nf, long long n,
+                                                               int first, double tol, MinresScalars* sc, int* flags,
+                                                               double* partials, unsigned* counter) {
+    if (!first && flags[0]) return;
+    double acc[1] = {0};
+    for_range(
+        nf, n,
+        [&](long long i) {
+            T z4[4], v4[4];
+            ld4(z + i, z4);
+            ld4(vv + i, v4);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[0] += double(z4[j]) * double(v4[j]);
+        },
+        [&](long long i) { acc[0] += double(z[i]) * double(vv[i]); });
+    grid_reduce<1>(acc, partials, counter, [&](double* tot) {
+        const double g2 = tot[0] + sc->dot;
+        if (first)
+            minres_start(sc, flags, g2, tol);
+        else
+            minres_scalars(sc, flags, g2);
+    });
+}
+
+template <typename T>
+__global__ void __launch_bounds__(VEC_THREADS) k_minres_step(MinresVecs<T> v, MinresScalars* sc, int* flags) {
+    if (!flags[1]) return;
+    const T zs = T(sc->zscale), a2 = T(sc->a2), a3 = T(sc->a3), ia1 = T(1.0 / sc->a1), xc = T(sc->xcoef);
+    for_range(
+        0, v.n,
+        [&](long long i) {
+            T z4[4], wo[4], wc[4], x4[4], wn[4];
+            ld4(v.z_cur + i, z4);
+            ld4(v.w_old + i, wo);
+            ld4(v.w_cur + i, wc);
+            ld4(v.x + i, x4);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                wn[j] = (z4[j] * zs - a3 * wo[j] - a2 * wc[j]) * ia1;
+                x4[j] += xc * wn[j];
+            }
+            st4(v.w_old + i, wn);
+            st4(v.x + i, x4);
+        },
+        [&](long long i) {
+            const T wn = (v.z_cur[i] * zs - a3 * v.w_old[i] - a2 * v.w_cur[i]) * ia1;
+            v.w_old[i] = wn;
+            v.x[i] += xc * wn;
+        });
+}
+
+__global__ void k_to_float(const double* in, float* out, double scale, long long n) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        out[i] = float(scale * in[i]);
+}
+
+__global__ void k_axpy_from_float(double* x, const float* d, double scale, long long n) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        x[i] += scale * double(d[i]);
+}
+
 // end of one body of the graph's while loop: continue while not converged and below the cap
 __global__ void k_loop_check(cudaGraphConditionalHandle h, const int* flags, int* loop) {
     int c = ++loop[0];
@@ -426,6 +621,63 @@ void cg_direction(CgVecs<T> v, Scalars* sc, int* flags, cudaStream_t s) {
 VG_CG_INSTANCES(double)
 VG_CG_INSTANCES(float)
 #undef VG_CG_INSTANCES
+
+template <typename T>
+void check_aligned(const MinresVecs<T>& v, const T* extra = nullptr) {
+    const void* ps[] = {v.v_cur, v.v_old, v.z_cur, v.z_new, v.w_cur, v.w_old, v.y, v.x, v.dinv, extra};
+    for (const void* p : ps)
+        if (reinterpret_cast<uintptr_t>(p) % 16) throw Error(VG_EINVAL, "Krylov vectors must be 16-byte aligned");
+}
+
+template <typename T>
+void minres_init(const T* r, MinresVecs<T> v, MinresScalars* sc, double* partials, unsigned* counter, cudaStream_t s) {
+    check_aligned(v, r);
+    k_minres_init<T><<<VEC_BLOCKS, VEC_THREADS, 0, s>>>(r, v, sc, partials, counter);
+    VG_CUDA(cudaGetLastError());
+}
+
+template <typename T>
+void minres_update(MinresVecs<T> v, bool flux, MinresScalars* sc, int* flags, double* partials, unsigned* counter,
+                   cudaStream_t s) {
+    if (flux)
+        k_minres_update<true, T><<<VEC_BLOCKS, VEC_THREADS, 0, s>>>(v, sc, flags, partials, counter);
+    else
+        k_minres_update<false, T><<<vec_blocks(v.n - v.nf), VEC_THREADS, 0, s>>>(v, sc, flags, partials, counter);
+    VG_CUDA(cudaGetLastError());
+}
+
+template <typename T>
+void minres_finish(const T* z, const T* v, long long nf, long long n, bool first, double tol, MinresScalars* sc,
+                   int* flags, double* partials, unsigned* counter, cudaStream_t s) {
+    k_minres_finish<T><<<VEC_BLOCKS, VEC_THREADS, 0, s>>>(z, v, nf, n, first, tol, sc, flags, partials, counter);
+    VG_CUDA(cudaGetLastError());
+}
+
+template <typename T>
+void minres_step(MinresVecs<T> v, MinresScalars* sc, int* flags, cudaStream_t s) {
+    k_minres_step<T><<<VEC_BLOCKS, VEC_THREADS, 0, s>>>(v, sc, flags);
+    VG_CUDA(cudaGetLastError());
+}
+
+#define VG_MINRES_INSTANCES(T)                                                                                      \
+    template void minres_init<T>(const T*, MinresVecs<T>, MinresScalars*, double*, unsigned*, cudaStream_t);        \
+    template void minres_update<T>(MinresVecs<T>, bool, MinresScalars*, int*, double*, unsigned*, cudaStream_t);    \
+    template void minres_finish<T>(const T*, const T*, long long, long long, bool, double, MinresScalars*, int*,    \
+                                   double*, unsigned*, cudaStream_t);                                               \
+    template void minres_step<T>(MinresVecs<T>, MinresScalars*, int*, cudaStream_t);
+VG_MINRES_INSTANCES(double)
+VG_MINRES_INSTANCES(float)
+#undef VG_MINRES_INSTANCES
+
+void to_float(const double* in, float* out, double scale, long long n, cudaStream_t s) {
+    k_to_float<<<vec_blocks(n), VEC_THREADS, 0, s>>>(in, out, scale, n);
+    VG_CUDA(cudaGetLastError());
+}
+
+void axpy_from_float(double* x, const float* d, double scale, long long n, cudaStream_t s) {
+    k_axpy_from_float<<<vec_blocks(n), VEC_THREADS, 0, s>>>(x, d, scale, n);
+    VG_CUDA(cudaGetLastError());
+}
 
 void loop_check(cudaGraphConditionalHandle h, const int* flags, int* loop, cudaStream_t s) {
     k_loop_check<<<1, 1, 0, s>>>(h, flags, loop);

@@ -81,6 +81,44 @@ void residual64(const double* b, const double* y, double* r, long long n, double
                 unsigned* counter, cudaStream_t s);
 // out = sign-flip of the pressure / multiplier block: out[i] = (i < nf ? 1 : -1) * in[i]
 void flip_pressure(const double* in, double* out, long long nf, long long n, cudaStream_t s);
+// ---- MINRES on the saddle-point form (vg_minres.cu) ----
+// scalars, device resident (double precision for both FP64 and FP32 inner solves)
+struct MinresScalars {
+    double gam_prev, gam, delta;   // gamma_{j-1}, gamma_j, raw z_j^T K z_j (from the apply)
+    double c_prev, c, s_prev, s;   // Givens c_{j-1}, c_j, s_{j-1}, s_j
+    double eta, eta0, tol;         // residual estimate |eta| (preconditioner norm), stop at tol * eta0
+    double a1, a2, a3, xcoef, zscale;
+    double dot;                    // z.v of the flux rows, until the pressure rows' share is known
+};
+// flags[0] = stop (converged or breakdown), flags[1] = current iteration valid, flags[2] = iterations
+
+// vectors of n entries, internal order: nf flux rows (dinv: their inverse diagonal), then pressure rows, whose part of
+// z is written by the V-cycle between the calls below
+template <typename T>
+struct MinresVecs {
+    T *v_cur, *v_old, *z_cur, *z_new, *w_cur, *w_old, *y, *x;
+    const T* dinv;
+    long long nf, n;
+};
+// v_cur = r, z = dinv r on the flux rows, everything else zero
+template <typename T>
+void minres_init(const T* r, MinresVecs<T> v, MinresScalars* sc, double* partials, unsigned* counter, cudaStream_t s);
+// v_new = y/g - (d/g) v_cur - (g/g_prev) v_old (into v_old), y = 0; flux: the flux rows, with z_new = dinv v_new and its
+// share of gamma^2; else the pressure rows
+template <typename T>
+void minres_update(MinresVecs<T> v, bool flux, MinresScalars* sc, int* flags, double* partials, unsigned* counter,
+                   cudaStream_t s);
+// the pressure rows' share of gamma^2 = z.v after the V-cycle, then the scalar recurrences (first: their start)
+template <typename T>
+void minres_finish(const T* z, const T* v, long long nf, long long n, bool first, double tol, MinresScalars* sc,
+                   int* flags, double* partials, unsigned* counter, cudaStream_t s);
+// w_new = (z_cur/g - a3 w_old - a2 w_cur)/a1 (into w_old), x += xcoef w_new
+template <typename T>
+void minres_step(MinresVecs<T> v, MinresScalars* sc, int* flags, cudaStream_t s);
+// out32 = float(scale in64); x64 += scale double(d32)
+void to_float(const double* in, float* out, double scale, long long n, cudaStream_t s);
+void axpy_from_float(double* x, const float* d, double scale, long long n, cudaStream_t s);
+
 // start of a solve: bs = r = b in the internal order (i2e) with the pressure and multiplier rows negated, x = 0 (null:
 // left alone), red[0] = red[1] = |b|^2 (deterministic)
 void start_residual(const double* b, const int* i2e, long long nf, long long n, double* bs, double* r, double* x,

@@ -281,6 +281,7 @@ Solver::Solver(HostMesh&& mesh, const vg_geometry* geo, int k_, int nq_, int ng_
 Solver::~Solver() {
     arena_.close();
     destroy_graphs();
+    destroy_minres_graphs();
     ms_destroy_graphs();
     if (h_err_) cudaFreeHost(h_err_);
     if (ev0_) cudaEventDestroy(ev0_);
@@ -467,6 +468,7 @@ void Solver::set_theta(const double* theta, bool on_device) {
                     d_A64_.data(), d_A32_.data(), nullptr);
         pack_streams(nullptr);
         pt.mark("rescale + record streams");
+        if (minres_.ready) prepare_minres();
         if (hybrid_ready_) prepare_hybrid();
         lift_flux_rhs();
         VG_CUDA(cudaDeviceSynchronize());
@@ -566,8 +568,8 @@ void Solver::build() {
     // a build starts the condensed system and its multigrid from scratch (the operator or the boundary
     // condition may have changed). With the pressure condition they are made here; with the flux condition
     // by the first solve, since a Maxwell-Stefan handle never needs them.
-    hybrid_condensed_ = hybrid_ready_ = use_amg = false;
-    if (bc == VG_BC_PRESSURE) prepare_hybrid();
+    hybrid_condensed_ = hybrid_ready_ = use_amg = minres_.ready = false;
+    if (bc == VG_BC_PRESSURE && !(minres_mesh() && prepare_minres())) prepare_hybrid();
     pt.mark("edge system (incl. multigrid)");
     // BC_FLUX: lifted right-hand side of MixedGpu::make_rhs (equation_gpu.cu:611-625):
     // free rows b - A g (unconstrained apply of the boundary values), boundary rows g
@@ -763,6 +765,8 @@ ApplyArgs<T> Solver::apply_args(const T* x, T* y, bool constrained, T psign, dou
     }
     return a;
 }
+template ApplyArgs<double> Solver::apply_args<double>(const double*, double*, bool, double, double*, const int*);
+template ApplyArgs<float> Solver::apply_args<float>(const float*, float*, bool, float, double*, const int*);
 
 void Solver::solve_host(const double* b_host, double* x_host, const vg_solve_opts& o, vg_solve_info& info) {
     if (!built) throw Error(VG_ESTATE, "vg_build must run before vg_solve_host");

@@ -7,6 +7,7 @@
 // Device side: FP64 setup outputs in bucket-slot-major layout (coalesced for one thread per
 // cell), FP64 and FP32 copies of the packed local operators, Krylov workspaces.
 #pragma once
+#include <functional>
 #include <memory>
 #include <string>
 #include <vector>
@@ -130,7 +131,34 @@ private:
     void prepare_condensation();
     void prepare_hybrid();
     std::vector<int> rank_order() const;  // rank of every cell
+    // graph Laplacian of the cells for one conductance per global edge; its values on the stored pattern of a hierarchy
+    // for conductances in the edges' own order
+    HostCsr cell_graph(const std::vector<double>& cond) const;
+    void laplacian_values(const Amg& amg, const double* cond, double* val);
     void build_amg();
+    // MINRES on the saddle-point form (vg_minres.cu)
+    bool minres_mesh() const;
+    bool prepare_minres();
+    template <typename T>
+    MinresVecs<T> minres_vecs();
+    template <typename T>
+    void minres_iteration(MinresVecs<T>& v, cudaStream_t s);
+    template <typename T>
+    void minres_build_graph(int p);
+    void destroy_minres_graphs();
+    template <typename T>
+    int minres_loop(const T* r, double tol, int maxit, int check_every, cudaStream_t s);
+    void minres_solve(double* x, const double* r, double nb, const vg_solve_opts& o,
+                      const std::function<double()>& residual, double& rel, int& total, int& outer, cudaStream_t s);
+    struct MinresState {
+        bool ready = false;
+        Amg amg;
+        DevBuf<double> w64[8], dinv64, cond, values, scal;
+        DevBuf<float> w32[8], dinv32, r32;
+        DevBuf<int> flags;
+        cudaGraph_t graph[2] = {nullptr, nullptr};
+        cudaGraphExec_t gexec[2] = {nullptr, nullptr};
+    } minres_;
     bool edges_planned_ = false, hybrid_planned_ = false, hybrid_condensed_ = false, hybrid_ready_ = false;
     std::vector<int> edge_order_;             // global edge -> index in the edge vectors
     DevBuf<int> d_emap_, d_rank_slot_;        // edge per (cell, local edge); slot of a cell's rank
