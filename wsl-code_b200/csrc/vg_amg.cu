@@ -126,17 +126,33 @@ double diag_of(const HostCsr& A, int i) {
     return 0.0;
 }
 
-// largest eigenvalue of D^{-1} A by power iteration (seeded start vector)
-double rho_dinv_a(const HostCsr& A, const std::vector<double>& dinv) {
-    int n = A.n;
-    std::vector<double> v(n), w(n);
+// Jacobi weight of the cycle over rho(D^{-1} A). The prolongator keeps the usual 4/3; as a smoother between the edge
+// interpolations 1.6 is better (with EDGE_RELAX, vg_krylov.cuh: 23 -> 20 iterations at 60k cells, lognormal K).
+constexpr double SMOOTH_WEIGHT = 1.6, PROLONG_WEIGHT = 4.0 / 3.0;
+// The cycle is definite only while the weight times rho(D^{-1} A) stays below 2, and a rough permeability takes rho from
+// 1.56 (uniform) to 2 on the finest level and beyond on the coarse ones. The power iteration's rho is an estimate from
+// below; the largest row sum of D^{-1} |A| is a bound. The finest level, where the bound is 2 and hardly above rho, has its
+// weight over it at most; the coarse levels, where it may be three times rho (1M cells: 43 iterations with it, 23 without),
+// only in a hierarchy made safe after a loop has met an indefinite cycle.
+constexpr double SAFE_WEIGHT = 1.9;
+constexpr int POWER_STEPS = 20;  // of the power iteration, on the host (setup) and on the device (refresh)
+
+std::vector<double> power_start(int n) {
+    std::vector<double> v(n);
     unsigned s = 12345u;
     for (int i = 0; i < n; ++i) {
         s = s * 1103515245u + 12345u;
         v[i] = 0.5 + (s >> 16) / 65536.0;
     }
+    return v;
+}
+
+// largest eigenvalue of D^{-1} A by power iteration (seeded start vector)
+double rho_dinv_a(const HostCsr& A, const std::vector<double>& dinv) {
+    int n = A.n;
+    std::vector<double> v = power_start(n), w(n);
     double lam = 1.0;
-    for (int it = 0; it < 20; ++it) {
+    for (int it = 0; it < POWER_STEPS; ++it) {
         double nv = 0;
         for (int i = 0; i < n; ++i) {
             double a = 0;
@@ -154,6 +170,17 @@ double rho_dinv_a(const HostCsr& A, const std::vector<double>& dinv) {
         for (int i = 0; i < n; ++i) v[i] = w[i] / nv;
     }
     return std::max(lam, 1e-300);
+}
+
+// a bound on it: the largest row sum of D^{-1} |A|
+double bound_dinv_a(const HostCsr& A, const std::vector<double>& dinv) {
+    double most = 0;
+    for (int i = 0; i < A.n; ++i) {
+        double s = 0;
+        for (int j = A.ptr[i]; j < A.ptr[i + 1]; ++j) s += std::fabs(A.val[j]);
+        most = std::max(most, s * std::fabs(dinv[i]));
+    }
+    return most;
 }
 
 // three-phase greedy aggregation on the strong-connection graph
@@ -261,10 +288,6 @@ HostCsr transfer_smooth(const HostCsr& P, const HostCsr& AP, const std::vector<d
 // device kernels (SELL-32, one thread per row)
 // ---------------------------------------------------------------------------------------------
 constexpr int TPB = 256;
-// Jacobi weight of the cycle over rho(D^{-1} A). The prolongator keeps the usual 4/3; as a smoother between the edge
-// interpolations 1.6 is better (with EDGE_RELAX, vg_krylov.cuh: 23 -> 20 iterations at 60k cells, lognormal K) and leaves
-// room below 2, where the cycle would stop being definite, for the power iteration's estimate of rho from below.
-constexpr double SMOOTH_WEIGHT = 1.6;
 constexpr int CSR_CAP = 2048;  // entries staged per CSR row block
 constexpr int CSR_RPT = 4;     // rows per thread of a CSR row block (at most CSR_RPT * TPB rows)
 
@@ -307,16 +330,16 @@ __device__ __forceinline__ T sell_finish(const DevSell<T>& M, const SellRow<T>& 
 // q = S (b + r). b is written by an earlier kernel: read with plain loads after the
 // programmatic-launch wait (never ld.global.nc, which the compiler may move above it)
 template <typename T>
-__global__ void __launch_bounds__(TPB) k_sell_residual(DevSell<T> A, const T* dinv, T omega, const T* b, T* q) {
+__global__ void __launch_bounds__(TPB) k_sell_residual(DevSell<T> A, const T* S, const T* b, T* q) {
     pdl_trigger();
     const int i = blockIdx.x * TPB + threadIdx.x;
     SellRow<T> R;
     if (i < A.n) sell_fetch<T>(A, i, R);
-    const T di = i < A.n ? __ldg(dinv + i) : T(0);
+    const T si = i < A.n ? __ldg(S + i) : T(0);
     pdl_wait();
     if (i < A.n) {
         const T bi = b[i], ri = bi - sell_finish<T>(A, R, b);
-        q[i] = omega * di * (bi + ri);
+        q[i] = si * (bi + ri);
     }
 }
 
@@ -331,7 +354,7 @@ __global__ void __launch_bounds__(TPB) k_sell_residual(DevSell<T> A, const T* di
 // by earlier kernels of the cycle are read with plain loads after the programmatic-launch wait
 // (never ld.global.nc, which the compiler may move above it); the matrix may be read before it.
 // op: 0 y = M x (restriction); 1 y = r + M x (prolongation, r holding S (b + residual) of the
-//     composite cycle); 2 y = omega dinv (b + (b - M x)) (that smoothed residual term, with x = b
+//     composite cycle); 2 y = S (b + (b - M x)) (that smoothed residual term, with x = b
 //     and M = A S)
 template <typename T>
 struct CsrSmem {
@@ -344,7 +367,7 @@ struct CsrSmem {
 };
 
 template <int OP, typename T, int LPR>
-__global__ void __launch_bounds__(TPB) k_csr(DevCsr<T> M, const T* dinv, T omega, const T* b, const T* x, T* y,
+__global__ void __launch_bounds__(TPB) k_csr(DevCsr<T> M, const T* S, const T* b, const T* x, T* y,
                                              const T* r) {
     // LPR threads per row: 1 (each thread sums up to CSR_RPT rows) or 8 for long rows (a row's
     // products summed by 8 threads, strided, then a fixed shuffle tree; at most TPB / 8 rows)
@@ -398,7 +421,7 @@ __global__ void __launch_bounds__(TPB) k_csr(DevCsr<T> M, const T* dinv, T omega
                     ep[q] = r[row];
                 else if (OP == 2) {
                     ep[q] = b[row];
-                    dd[q] = __ldg(dinv + row);
+                    dd[q] = __ldg(S + row);
                 }
             }
         }
@@ -475,7 +498,7 @@ __global__ void __launch_bounds__(TPB) k_csr(DevCsr<T> M, const T* dinv, T omega
                 y[row] = ep[q] + acc[q];
             else {
                 const T rr = ep[q] - acc[q];
-                y[row] = omega * dd[q] * (ep[q] + rr);
+                y[row] = dd[q] * (ep[q] + rr);
             }
         }
     }
@@ -490,7 +513,7 @@ __global__ void __launch_bounds__(TPB) k_csr(DevCsr<T> M, const T* dinv, T omega
 // warp from global memory (strided partial sums, fixed shuffle tree). Same ops as k_csr.
 constexpr int WS_CAP = 128, WS_J = WS_CAP / 32, WS_WARPS = 8;
 template <int OP, typename T, int LPR>
-__global__ void __launch_bounds__(WS_WARPS * 32) k_csr_ws(DevCsr<T> M, const T* dinv, T omega, const T* b,
+__global__ void __launch_bounds__(WS_WARPS * 32) k_csr_ws(DevCsr<T> M, const T* S, const T* b,
                                                           const T* x, T* y, const T* r) {
     __shared__ T prod[WS_WARPS][WS_CAP];
     pdl_trigger();
@@ -519,7 +542,7 @@ __global__ void __launch_bounds__(WS_WARPS * 32) k_csr_ws(DevCsr<T> M, const T* 
         c[j] = in ? __ldg(M.col + a.y + k) : 0;
         v[j] = in ? __ldg(M.val + a.y + k) : T(0);
     }
-    const T dl = (OP == 2 && rl) ? __ldg(dinv + row) : T(0);
+    const T dl = (OP == 2 && rl) ? __ldg(S + row) : T(0);
     pdl_wait();
     if (!live) return;
     T ep = T(0);
@@ -557,7 +580,7 @@ __global__ void __launch_bounds__(WS_WARPS * 32) k_csr_ws(DevCsr<T> M, const T* 
             y[row] = ep + acc;
         else {
             const T rr = ep - acc;
-            y[row] = omega * dl * (ep + rr);
+            y[row] = dl * (ep + rr);
         }
     }
 }
@@ -595,7 +618,7 @@ void prepare_csr_kernels(int slots[2]) {
 }
 
 template <typename T>
-void launch_csr(int op, const DevCsr<T>& M, const T* dinv, T omega, const T* b, const T* x, T* y, const T* r,
+void launch_csr(int op, const DevCsr<T>& M, const T* S, const T* b, const T* x, T* y, const T* r,
                 cudaStream_t s) {
     if (M.n <= 0 || M.nblk <= 0) return;
     const int grid = std::min(M.nblk, std::max(1, M.slots));
@@ -603,48 +626,48 @@ void launch_csr(int op, const DevCsr<T>& M, const T* dinv, T omega, const T* b, 
     switch (op) {
     case 0:
         if (M.lpr > 1)
-            launch_pdl(k_csr<0, T, 8>, grid, TPB, sb, s, M, dinv, omega, b, x, y, r);
+            launch_pdl(k_csr<0, T, 8>, grid, TPB, sb, s, M, S, b, x, y, r);
         else
-            launch_pdl(k_csr<0, T, 1>, grid, TPB, sb, s, M, dinv, omega, b, x, y, r);
+            launch_pdl(k_csr<0, T, 1>, grid, TPB, sb, s, M, S, b, x, y, r);
         break;
     case 1:
         if (M.lpr > 1)
-            launch_pdl(k_csr<1, T, 8>, grid, TPB, sb, s, M, dinv, omega, b, x, y, r);
+            launch_pdl(k_csr<1, T, 8>, grid, TPB, sb, s, M, S, b, x, y, r);
         else
-            launch_pdl(k_csr<1, T, 1>, grid, TPB, sb, s, M, dinv, omega, b, x, y, r);
+            launch_pdl(k_csr<1, T, 1>, grid, TPB, sb, s, M, S, b, x, y, r);
         break;
     default:
         if (M.lpr > 1)
-            launch_pdl(k_csr<2, T, 8>, grid, TPB, sb, s, M, dinv, omega, b, x, y, r);
+            launch_pdl(k_csr<2, T, 8>, grid, TPB, sb, s, M, S, b, x, y, r);
         else
-            launch_pdl(k_csr<2, T, 1>, grid, TPB, sb, s, M, dinv, omega, b, x, y, r);
+            launch_pdl(k_csr<2, T, 1>, grid, TPB, sb, s, M, S, b, x, y, r);
         break;
     }
 }
 
 template <typename T>
-void launch_ws(int op, const DevCsr<T>& M, const T* dinv, T omega, const T* b, const T* x, T* y, const T* r,
+void launch_ws(int op, const DevCsr<T>& M, const T* S, const T* b, const T* x, T* y, const T* r,
                cudaStream_t s) {
     if (M.n <= 0 || M.nwb <= 0) return;
     const int grid = (M.nwb + WS_WARPS - 1) / WS_WARPS;
     switch (op) {
     case 0:
         if (M.lpr > 1)
-            launch_pdl(k_csr_ws<0, T, 8>, grid, WS_WARPS * 32, 0, s, M, dinv, omega, b, x, y, r);
+            launch_pdl(k_csr_ws<0, T, 8>, grid, WS_WARPS * 32, 0, s, M, S, b, x, y, r);
         else
-            launch_pdl(k_csr_ws<0, T, 1>, grid, WS_WARPS * 32, 0, s, M, dinv, omega, b, x, y, r);
+            launch_pdl(k_csr_ws<0, T, 1>, grid, WS_WARPS * 32, 0, s, M, S, b, x, y, r);
         break;
     case 1:
         if (M.lpr > 1)
-            launch_pdl(k_csr_ws<1, T, 8>, grid, WS_WARPS * 32, 0, s, M, dinv, omega, b, x, y, r);
+            launch_pdl(k_csr_ws<1, T, 8>, grid, WS_WARPS * 32, 0, s, M, S, b, x, y, r);
         else
-            launch_pdl(k_csr_ws<1, T, 1>, grid, WS_WARPS * 32, 0, s, M, dinv, omega, b, x, y, r);
+            launch_pdl(k_csr_ws<1, T, 1>, grid, WS_WARPS * 32, 0, s, M, S, b, x, y, r);
         break;
     default:
         if (M.lpr > 1)
-            launch_pdl(k_csr_ws<2, T, 8>, grid, WS_WARPS * 32, 0, s, M, dinv, omega, b, x, y, r);
+            launch_pdl(k_csr_ws<2, T, 8>, grid, WS_WARPS * 32, 0, s, M, S, b, x, y, r);
         else
-            launch_pdl(k_csr_ws<2, T, 1>, grid, WS_WARPS * 32, 0, s, M, dinv, omega, b, x, y, r);
+            launch_pdl(k_csr_ws<2, T, 1>, grid, WS_WARPS * 32, 0, s, M, S, b, x, y, r);
         break;
     }
 }
@@ -655,12 +678,12 @@ void launch_ws(int op, const DevCsr<T>& M, const T* dinv, T omega, const T* b, c
 // restrictions, the denser coarse operators) are summed by 8 threads per row in both kernels
 // (mixed 14.31 -> 14.13 ms, FP64 21.49 -> 21.14 ms)
 template <typename T>
-void launch_prod(int op, const DevCsr<T>& M, const T* dinv, T omega, const T* b, const T* x, T* y, const T* r,
+void launch_prod(int op, const DevCsr<T>& M, const T* S, const T* b, const T* x, T* y, const T* r,
                  cudaStream_t s) {
     if constexpr (sizeof(T) == 8)
-        launch_ws<T>(op, M, dinv, omega, b, x, y, r, s);
+        launch_ws<T>(op, M, S, b, x, y, r, s);
     else
-        launch_csr<T>(op, M, dinv, omega, b, x, y, r, s);
+        launch_csr<T>(op, M, S, b, x, y, r, s);
 }
 
 // coarsest level: z = Ainv b, one warp per row. The inverse does not change between cycles: its
@@ -910,27 +933,84 @@ __device__ __forceinline__ int find_col(const int* col, int lo, int hi, int c) {
     return lo;  // position of c when present
 }
 
-__global__ void k_diag_inv(const int* ptr, const int* col, const double* val, int n, double* d64, float* d32) {
-    int r = blockIdx.x * TPB + threadIdx.x;
-    if (r >= n) return;
-    int lo = ptr[r], hi = ptr[r + 1];
-    int j = find_col(col, lo, hi, r);
-    double v = (j < hi && col[j] == r) ? val[j] : 0.0;
-    double iv = v != 0.0 ? 1.0 / v : 0.0;
-    d64[r] = iv;
-    d32[r] = float(iv);
+// a level's rho(D^{-1} A): rho[0] the estimate, rho[1] the bound or 0 where it is not asked for
+__device__ __forceinline__ double jacobi_weight(double w, const double* rho) {
+    return fmin(w / rho[0], SAFE_WEIGHT / rho[1]);
+}
+
+// D^{-1}, and with bound the largest row sum of D^{-1} |A| (zero on entry; positive doubles compare like their bits)
+__global__ void k_diag_inv(const int* ptr, const int* col, const double* val, int n, double* dinv, double* bound) {
+    const int r = blockIdx.x * TPB + threadIdx.x;
+    double sum = 0.0;
+    if (r < n) {
+        const int lo = ptr[r], hi = ptr[r + 1], j = find_col(col, lo, hi, r);
+        const double v = (j < hi && col[j] == r) ? val[j] : 0.0, iv = v != 0.0 ? 1.0 / v : 0.0;
+        dinv[r] = iv;
+        for (int e = lo; e < hi; ++e) sum += fabs(val[e]);
+        sum *= fabs(iv);
+    }
+    if (!bound) return;
+    for (int o = 16; o; o >>= 1) sum = fmax(sum, __shfl_down_sync(0xffffffffu, sum, o));
+    if ((threadIdx.x & 31) == 0)
+        atomicMax(reinterpret_cast<unsigned long long*>(bound), (unsigned long long)__double_as_longlong(sum));
+}
+
+// w = D^{-1} A v, eight lanes a row
+__global__ void __launch_bounds__(TPB) k_power(const int* ptr, const int* col, const double* val, const double* dinv, int n,
+                                               const double* v, double* w) {
+    const int r = (blockIdx.x * TPB + threadIdx.x) / 8, sub = threadIdx.x % 8;
+    double s = 0.0;
+    if (r < n)
+        for (int j = ptr[r] + sub; j < ptr[r + 1]; j += 8) s += val[j] * v[col[j]];
+    for (int o = 4; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, 8);
+    if (r < n && sub == 0) w[r] = dinv[r] * s;
+}
+
+// the power iteration's estimate (w, v) / (v, v), one CTA, fixed order
+__global__ void __launch_bounds__(1024) k_rayleigh(const double* w, const double* v, int n, double* rho) {
+    __shared__ double sh[2][32];
+    double a = 0.0, b = 0.0;
+    for (int i = threadIdx.x; i < n; i += 1024) {
+        a += w[i] * v[i];
+        b += v[i] * v[i];
+    }
+    for (int o = 16; o; o >>= 1) {
+        a += __shfl_down_sync(0xffffffffu, a, o);
+        b += __shfl_down_sync(0xffffffffu, b, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        sh[0][threadIdx.x >> 5] = a;
+        sh[1][threadIdx.x >> 5] = b;
+    }
+    __syncthreads();
+    if (threadIdx.x) return;
+    a = b = 0.0;
+    for (int i = 0; i < 32; ++i) {
+        a += sh[0][i];
+        b += sh[1][i];
+    }
+    *rho = fmax(a / b, 1e-300);
+}
+
+// S = smooth D^{-1} in both precisions
+__global__ void k_smoother(const double* dinv, double weight, const double* rho, int n, double* s64, float* s32) {
+    const int i = blockIdx.x * TPB + threadIdx.x;
+    if (i >= n) return;
+    const double w = jacobi_weight(weight, rho);
+    s64[i] = w * dinv[i];
+    s32[i] = float(w) * float(dinv[i]);
 }
 
 // P = (I - omega D^{-1} A) P_tent on the fixed pattern of P (rows in A's stored order)
 __global__ void k_smooth_p(const int* aptr, const int* acol, const double* aval, const int* agg, const double* dinv,
-                           double omega, const int* pptr, const int* pcol, double* pval, int n) {
+                           const double* rho, const int* pptr, const int* pcol, double* pval, int n) {
     int t = blockIdx.x * TPB + threadIdx.x;
     if (t >= n) return;
     const int lo = pptr[t], hi = pptr[t + 1];
     for (int j = lo; j < hi; ++j) pval[j] = 0.0;
     int j = find_col(pcol, lo, hi, agg[t]);
     if (j < hi && pcol[j] == agg[t]) pval[j] += 1.0;
-    const double f = -omega * dinv[t];
+    const double f = -jacobi_weight(PROLONG_WEIGHT, rho) * dinv[t];
     for (int e = aptr[t]; e < aptr[t + 1]; ++e) {
         const int J = agg[acol[e]];
         j = find_col(pcol, lo, hi, J);
@@ -961,9 +1041,9 @@ __global__ void k_rap(const int* rptr, const int* rcol, const double* rval, cons
     cval[z] = s;
 }
 
-// A P and Pt = (I - omega D^{-1} A) P on Pt's fixed pattern, one entry (t, J) per thread: A's row t in order, column J
-// of P's rows found by bisection, then Pt = P - omega d_t (A P)
-__global__ void k_ptilde(const int* aptr, const int* acol, const double* aval, const double* dinv, double omega,
+// A P and Pt = (I - S A) P on Pt's fixed pattern, one entry (t, J) per thread: A's row t in order, column J
+// of P's rows found by bisection, then Pt = P - S_t (A P)
+__global__ void k_ptilde(const int* aptr, const int* acol, const double* aval, const double* S,
                          const int* pptr, const int* pcol, const double* pval, const int* qrow, const int* qcol,
                          double* apval, double* qval, long long nnz) {
     const long long z = blockIdx.x * (long long)TPB + threadIdx.x;
@@ -976,7 +1056,7 @@ __global__ void k_ptilde(const int* aptr, const int* acol, const double* aval, c
     double s = 0.0;
     for (int e = aptr[t]; e < aptr[t + 1]; ++e) s += aval[e] * p_of(acol[e]);
     apval[z] = s;
-    qval[z] = p_of(t) - omega * dinv[t] * s;
+    qval[z] = p_of(t) - S[t] * s;
 }
 
 // row of every stored entry
@@ -985,12 +1065,12 @@ __global__ void k_expand_rows(const int* ptr, int n, int* row) {
         for (int j = ptr[r]; j < ptr[r + 1]; ++j) row[j] = r;
 }
 
-// values of A S (columns scaled by omega D^{-1}) from A's stored CSR values, into CSR (pos null)
+// values of A S from A's stored CSR values, into CSR (pos null)
 // or SELL slots
-__global__ void k_scale_cols(const double* aval, const int* acol, const double* dinv, double omega,
+__global__ void k_scale_cols(const double* aval, const int* acol, const double* S,
                              const long long* pos, double* out, long long n) {
     for (long long i = blockIdx.x * (long long)TPB + threadIdx.x; i < n; i += (long long)gridDim.x * TPB) {
-        const double v = aval[i] * (omega * dinv[acol[i]]);
+        const double v = aval[i] * S[acol[i]];
         out[pos ? pos[i] : i] = v;
     }
 }
@@ -1081,17 +1161,20 @@ void Amg::release_streams() {
     side_ = nullptr;
 }
 
-void Amg::refresh(const double* a0) {
+void Amg::refresh(const double* a0, bool safe) {
     if (levels_.empty()) throw Error(VG_ESTATE, "multigrid refresh before setup");
     PhaseTimer pt;
     const int nl = int(levels_.size());
     const double* aval = a0;
+    if (!rho_.data()) {
+        std::vector<double> rho(2 * size_t(nl), 0.0);
+        rho[0] = levels_[0].rho;
+        rho_.upload(rho);
+    }
     for (int l = 0; l < nl; ++l) {
         Level& L = levels_[l];
         const long long nnz = (long long)L.pa_col.size();
-        k_diag_inv<<<blocks(L.n), TPB>>>(L.dpa_ptr.data(), L.dpa_col.data(), aval, L.n, L.dinv64.data(),
-                                         L.dinv32.data());
-        VG_CUDA(cudaGetLastError());
+        double* const rho = rho_.data() + 2 * l;
         if (l == nl - 1) {  // coarsest: dense inverse of the refreshed matrix
             if (pt.on) VG_CUDA(cudaDeviceSynchronize());
             pt.mark("refresh: levels");
@@ -1099,19 +1182,35 @@ void Amg::refresh(const double* a0) {
             pt.mark("refresh: coarsest inverse");
             break;
         }
+        VG_CUDA(cudaMemsetAsync(rho + 1, 0, sizeof(double), nullptr));
+        k_diag_inv<<<blocks(L.n), TPB>>>(L.dpa_ptr.data(), L.dpa_col.data(), aval, L.n, L.dinv64.data(),
+                                         l == 0 || safe ? rho + 1 : nullptr);
+        if (l > 0) {  // as setup() does (without its scaling of the iterates, which rho^20 does not need)
+            const double* v = L.power.data();
+            double *w = L.x64.data(), *free = L.r64.data();
+            for (int it = 0; it < POWER_STEPS; ++it) {
+                if (it) {
+                    v = w;
+                    std::swap(w, free);
+                }
+                k_power<<<blocks(8 * L.n), TPB>>>(L.dpa_ptr.data(), L.dpa_col.data(), aval, L.dinv64.data(), L.n, v, w);
+            }
+            k_rayleigh<<<1, 1024>>>(w, v, L.n, rho);
+        }
+        k_smoother<<<blocks(L.n), TPB>>>(L.dinv64.data(), saddle_ ? PROLONG_WEIGHT : SMOOTH_WEIGHT, rho, L.n,
+                                         L.s64.data(), L.s32.data());
         // A S for the residual
         if (L.A.csr) {
-            k_scale_cols<<<148 * 4, TPB>>>(aval, L.dpa_col.data(), L.dinv64.data(), L.smooth, nullptr, L.cA.v64.data(),
-                                           nnz);
+            k_scale_cols<<<148 * 4, TPB>>>(aval, L.dpa_col.data(), L.s64.data(), nullptr, L.cA.v64.data(), nnz);
             k_to32<<<148 * 4, TPB>>>(L.cA.v64.data(), L.cA.v32.data(), nnz);
         } else {
-            k_scale_cols<<<148 * 4, TPB>>>(aval, L.dpa_col.data(), L.dinv64.data(), L.smooth, L.dsellpos.data(),
-                                           L.dA_v64.data(), nnz);
+            k_scale_cols<<<148 * 4, TPB>>>(aval, L.dpa_col.data(), L.s64.data(), L.dsellpos.data(), L.dA_v64.data(),
+                                           nnz);
             k_to32<<<148 * 4, TPB>>>(L.dA_v64.data(), L.dA_v32.data(), (long long)L.dA_v64.size());
         }
         // P, R = P^T (FP64: the next level's Galerkin product), Pt = (I - S A) P and Rt = Pt^T
         k_smooth_p<<<blocks(L.n), TPB>>>(L.dpa_ptr.data(), L.dpa_col.data(), aval, L.dagg.data(), L.dinv64.data(),
-                                         L.omega, L.cP.ptr.data(), L.cP.col.data(), L.cP.v64.data(), L.n);
+                                         rho, L.cP.ptr.data(), L.cP.col.data(), L.cP.v64.data(), L.n);
         k_take<<<148 * 4, TPB>>>(L.cP.v64.data(), L.dr2p.data(), L.cR.v64.data(), (long long)L.r2p.size());
         const long long ptn = (long long)L.rt2pt.size();
         Level& C = levels_[l + 1];
@@ -1123,7 +1222,7 @@ void Amg::refresh(const double* a0) {
             k_expand_rows<<<blocks(L.n), TPB>>>(L.cPt.ptr.data(), L.n, L.dpt_row.data());
             k_expand_rows<<<blocks(C.n), TPB>>>(C.dpa_ptr.data(), C.n, C.dpa_row.data());
         }
-        k_ptilde<<<int((ptn + TPB - 1) / TPB), TPB>>>(L.dpa_ptr.data(), L.dpa_col.data(), aval, L.dinv64.data(), L.smooth,
+        k_ptilde<<<int((ptn + TPB - 1) / TPB), TPB>>>(L.dpa_ptr.data(), L.dpa_col.data(), aval, L.s64.data(),
                                                       L.cP.ptr.data(), L.cP.col.data(), L.cP.v64.data(),
                                                       L.dpt_row.data(), L.cPt.col.data(), L.dap.data(),
                                                       L.cPt.v64.data(), ptn);
@@ -1152,6 +1251,7 @@ void Amg::setup(const HostCsr& S0, int* err, const std::vector<int>* fine_order,
     constant_kernel_ = constant_kernel;
     saddle_ = saddle;
     levels_.clear();
+    rho_.resize(0);
     release_streams();
     HostCsr A = S0;
     const double theta = 0.08;
@@ -1266,7 +1366,9 @@ void Amg::setup(const HostCsr& S0, int* err, const std::vector<int>* fine_order,
             } else {
                 const double rho = rho_dinv_a(A, dinv_own);
                 L.omega = 4.0 / (3.0 * rho);
+                L.rho = rho;
                 L.smooth = saddle ? L.omega : SMOOTH_WEIGHT / rho;
+                if (!saddle && levels_.empty()) L.smooth = std::min(L.smooth, SAFE_WEIGHT / bound_dinv_a(A, dinv_own));
                 P = smoothed_prolongator(A, agg, nagg, dinv_own, L.omega);
                 L.agg.resize(A.n);
                 for (int i = 0; i < A.n; ++i) L.agg[fine ? (*fine_order)[i] : i] = agg[i];
@@ -1357,9 +1459,18 @@ void Amg::setup(const HostCsr& S0, int* err, const std::vector<int>* fine_order,
         L.dpa_ptr.upload(L.pa_ptr);
         L.dpa_col.upload(L.pa_col);
         if (l > 0) L.dvals.resize(L.pa_col.size());  // written by refresh()
-        L.dinv64.upload(L.dinv);
-        std::vector<float> f(L.dinv.begin(), L.dinv.end());
-        L.dinv32.upload(f);
+        L.dinv64.resize(L.n);  // written by refresh()
+        if (!coarsest) {
+            std::vector<double> s64(L.n);
+            std::vector<float> s32(L.n);
+            for (int i = 0; i < L.n; ++i) {
+                s64[i] = L.smooth * L.dinv[i];
+                s32[i] = float(L.smooth) * float(L.dinv[i]);
+            }
+            if (l > 0) L.power.upload(power_start(L.n));
+            L.s64.upload(s64);
+            L.s32.upload(s32);
+        }
         for (auto* b : {&L.x64, &L.b64, &L.r64}) b->resize(L.n);
         for (auto* b : {&L.x32, &L.b32, &L.r32}) b->resize(L.n);
     }
@@ -1450,8 +1561,7 @@ bool Amg::view_levels(AmgView<T>& out) {
         v.pptr = L.cPt.ptr.data();
         v.pcol = L.cPt.col.data();
         v.pval = pick(L.cPt.v64, L.cPt.v32);
-        v.dinv = pick(L.dinv64, L.dinv32);
-        v.omega = T(L.smooth);
+        v.S = pick(L.s64, L.s32);
         v.a_wide = L.pa_col.size() >= 10 * size_t(L.n);
         v.r_wide = L.rt2pt.size() >= 10 * size_t(L.nc);
         v.p_wide = L.rt2pt.size() >= 10 * size_t(L.n);
@@ -1485,21 +1595,21 @@ void Amg::cycle(int l, const T* b, T* z, cudaStream_t s) {
         return;
     }
     Level& C = levels_[l + 1];
-    const T* dinv = buf(L.dinv64, L.dinv32);
+    const T* S = buf(L.s64, L.s32);
     T* r = buf(L.r64, L.r32);
     T* bc = buf(C.b64, C.b32);
     T* xc = buf(C.x64, C.x32);
     VG_CUDA(cudaEventRecord(ev_fork_[l], s));
     VG_CUDA(cudaStreamWaitEvent(side_, ev_fork_[l], 0));
     if (L.A.csr)
-        launch_prod<T>(2, cview<T>(L.A, L.cA), dinv, T(L.smooth), b, b, r, nullptr, side_);
+        launch_prod<T>(2, cview<T>(L.A, L.cA), S, b, b, r, nullptr, side_);
     else
-        launch_pdl(k_sell_residual<T>, blocks(L.n), TPB, 0, side_, view<T>(L), dinv, T(L.smooth), b, r);
+        launch_pdl(k_sell_residual<T>, blocks(L.n), TPB, 0, side_, view<T>(L), S, b, r);
     VG_CUDA(cudaEventRecord(ev_join_[l], side_));
-    launch_prod<T>(0, cview<T>(L.Rt, L.cRt), nullptr, T(0), nullptr, b, bc, nullptr, s);
+    launch_prod<T>(0, cview<T>(L.Rt, L.cRt), nullptr, nullptr, b, bc, nullptr, s);
     cycle<T>(l + 1, bc, xc, s);
     VG_CUDA(cudaStreamWaitEvent(s, ev_join_[l], 0));
-    launch_prod<T>(1, cview<T>(L.Pt, L.cPt), dinv, T(L.smooth), b, xc, z, r, s);
+    launch_prod<T>(1, cview<T>(L.Pt, L.cPt), S, b, xc, z, r, s);
     launches += 3;
 }
 

@@ -64,8 +64,7 @@ struct AmgLevelView {
     const int *aptr, *acol;
     const T* aval;
     const int *rptr, *rcol, *pptr, *pcol;  // Rt, Pt
-    const T *rval, *pval, *dinv;
-    T omega;
+    const T *rval, *pval, *S;
     bool a_wide, r_wide, p_wide;   // rows of ten entries and more on average
     T *r, *b, *x;                  // this level's smoothed residual; the next level's right-hand side and solution
 };
@@ -109,10 +108,12 @@ public:
     template <typename T>
     bool view_levels(AmgView<T>& out);
     // Recompute every value of the hierarchy on the device for a new finest-level operator with the
-    // same sparsity: the aggregates, sparsity patterns and smoothing weights of setup() are kept
-    // (a valid multigrid for any values; the captured cycle's device addresses do not change).
+    // same sparsity: the aggregates and sparsity patterns of setup() are kept, the weights follow the new values'
+    // rho(D^{-1} A) (a bound on it on the finest level, an estimate on the others; the captured cycle's device addresses
+    // do not change).
     // a0: the finest level's values in the order of its stored pattern (level0_ptr / level0_col).
-    void refresh(const double* a0);
+    // safe: every level's weights held below the bound.
+    void refresh(const double* a0, bool safe = false);
     const int* level0_ptr() const { return levels_.empty() ? nullptr : levels_[0].dpa_ptr.data(); }
     const int* level0_col() const { return levels_.empty() ? nullptr : levels_[0].dpa_col.data(); }
     long long level0_nnz() const { return levels_.empty() ? 0 : (long long)levels_[0].pa_col.size(); }
@@ -139,6 +140,7 @@ private:
     struct Level {
         int n = 0, nc = 0;
         double omega = 0;   // prolongator smoothing, 4 / (3 rho(D^{-1} A))
+        double rho = 0;     // the estimate of rho(D^{-1} A) that both come from
         double smooth = 0;  // the cycle's Jacobi smoothing, SMOOTH_WEIGHT / rho
         // A: the level's operator with its columns scaled by S = smooth D^{-1} (A S, for the residual
         // r = b - A S b); Pt = (I - S A) P: n x nc, Rt = Pt^T: nc x n (absent on the coarsest level)
@@ -161,8 +163,9 @@ private:
         DevBuf<double> dA_v64;
         DevBuf<float> dA_v32;
         CsrBufs cA, cPt, cRt;
-        DevBuf<double> dinv64, x64, b64, r64;
-        DevBuf<float> dinv32, x32, b32, r32;
+        DevBuf<double> power;  // start of the power iteration (refresh)
+        DevBuf<double> dinv64, s64, x64, b64, r64;  // s: S = smooth D^{-1}
+        DevBuf<float> s32, x32, b32, r32;
     };
     template <typename T>
     void cycle(int l, const T* b, T* z, cudaStream_t s);
@@ -176,6 +179,7 @@ private:
     std::vector<Level> levels_;
     int ncoarse_ = 0;
     bool constant_kernel_ = false, saddle_ = false;
+    DevBuf<double> rho_;  // refresh: rho(D^{-1} A) of every level, estimate and bound
     int* err_ = nullptr;  // the owner's error word: set when a cycle kernel gave up on a copy (never in a correct run)
     int csr_slots_[2] = {1, 1};  // resident CTAs of the CSR kernels on this hierarchy's device (FP32, FP64)
     DevBuf<double> dinvc64_;  // dense inverse of the coarsest matrix

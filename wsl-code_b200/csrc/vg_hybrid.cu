@@ -575,7 +575,18 @@ void Solver::prepare_hybrid() {
         build_amg();
         pt.mark("multigrid");
     }
+    amg_safe_ = false;
     hybrid_ready_ = true;
+}
+
+// every weight of the current hierarchy below the bound that keeps the cycle definite, until the next update
+void Solver::make_amg_safe() {
+    ArenaScope scope(arena_);
+    VG_CUDA(cudaStreamSynchronize(stream_));
+    d_lap_.resize(size_t(amg_.level0_nnz()));
+    laplacian_values(amg_, d_econd_.data(), d_lap_.data());
+    amg_.refresh(d_lap_.data(), true);
+    amg_safe_ = true;
 }
 
 std::vector<int> Solver::rank_order() const {
@@ -971,6 +982,21 @@ void Solver::solve(const double* b, double* x, const vg_solve_opts& o, vg_solve_
         int it = 0;
         const double gain = finish_correction(out, it);
         total += it;
+        // r.z not positive: the cycle, whose coarse levels have estimated weights, is not definite on these values. The
+        // hierarchy is made safe, and a correction that did harm is taken back.
+        if (rel > o.tol && use_amg && !amg_safe_ && !(out.sc.rz > 0 && out.sc.rz0 > 0)) {
+            make_amg_safe();
+            if (!(rel < before)) {
+                if (direct)
+                    VG_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * N, s));
+                else
+                    axpy64(x, d.data(), -1.0, s);
+                true_residual();
+                rel = read();
+                n_launch += 1;
+            }
+            continue;
+        }
         if (!direct) ratio = std::min(1e8, std::max(1.0, rel / (before * gain)));
         idle = rel <= 0.5 * before ? 0 : idle + 1;
         if (fp64 && idle >= 3) {  // rounding level

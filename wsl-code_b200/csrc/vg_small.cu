@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(ST, 1) k_small_cg(SmallCg<T> a) {
             row_sums(Rt[l], A.r_wide, b, [&](int row, T s) { A.b[row] = s; });
             auto smooth = [&](int row, T s) {
                 const T bi = b[row];
-                A.r[row] = A.omega * __ldg(A.dinv + row) * (bi + (bi - s));
+                A.r[row] = __ldg(A.S + row) * (bi + (bi - s));
             };
             if (As[l].local || !A.sell.val)
                 row_sums(As[l], A.a_wide, b, smooth);

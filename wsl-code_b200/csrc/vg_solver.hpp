@@ -136,6 +136,8 @@ private:
     HostCsr cell_graph(const std::vector<double>& cond) const;
     void laplacian_values(const Amg& amg, const double* cond, double* val);
     void build_amg();
+    void make_amg_safe();
+    bool amg_safe_ = false;
     // MINRES on the saddle-point form (vg_minres.cu)
     bool minres_mesh() const;
     bool prepare_minres();
