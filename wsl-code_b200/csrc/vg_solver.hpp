@@ -204,9 +204,9 @@ private:
         long long N = 0, n = 0;  // state, edge system (2 per edge)
         DevBuf<double> B64, m64, b, r, y, d;  // friction, |E|/dt; state vectors of a step
         DevBuf<float> B32, m32, A32;
-        DevBuf<double> prev;  // Picard: the iterate the friction matrix was taken at
+        DevBuf<double> prev, first;  // Picard: the iterate the friction matrix was taken at; the old state
         // edge system: cells' condensed values, 2 x 2 blocks, preconditioner blocks and weights
-        DevBuf<double> S64, Y64, tsum, c64, D, Di64, lam, res, cw64, ew64, rc64[2], zc64[2];
+        DevBuf<double> S64, Y64, c64, D, Di64, G, Gi, res, cw64, ew64, rc64[2], zc64[2];
         DevBuf<float> S32, Y32, c32, Di32, cw32, ew32, rc32[2], zc32[2];
         DevBuf<double> V64, h, r64, l64, t64, w64, vn64, partials, kry;
         DevBuf<float> V32, r32, l32, t32, w32, vn32;
