@@ -949,10 +949,11 @@ void Solver::solve(const double* b, double* x, const vg_solve_opts& o, vg_solve_
     // one FP64 loop spares a second launch, its set-up and the residual between (mixed with FP32 loops -> with this one,
     // us: 100 cells 328 -> 263, 1,000 386 -> 305, 8,000 549 -> 452, 45,000 923 -> 806). From degree 1 on the FP64
     // blocks cost what they spare (10,000 cells 981 against 1,052, degree 2 40,000 cells 14,851 against 16,482).
-    const bool fp64 = o.mode == VG_SOLVE_FP64 || (k == 0 && o.check_every <= 0 && takes_one_launch<double>());
+    bool fp64 = o.mode == VG_SOLVE_FP64 || (k == 0 && o.check_every <= 0 && takes_one_launch<double>());
     const int steps = minres_.ready ? 0 : o.mode == VG_SOLVE_FP64 ? 12 : o.max_outer;
     double ratio = 1.0;
     int idle = 0;
+    bool careful = false;  // loops end after six digits
     for (; outer < steps && rel > o.tol && total < o.maxit; ++outer) {
         const double want = 0.1 * o.tol / (rel * ratio), before = rel;
         CgStop stop;
@@ -965,7 +966,7 @@ void Solver::solve(const double* b, double* x, const vg_solve_opts& o, vg_solve_
         if (fp64) {
             stop.unit = 0.0;
             stop.tol = std::min(0.5, want);
-            stop.floor = 1e-15;
+            stop.floor = careful ? 1e-6 : 1e-15;
             correct<double>(r.data(), to, stop, o.maxit - total, o.check_every, s);
         } else {
             stop.unit = rel;
@@ -982,10 +983,11 @@ void Solver::solve(const double* b, double* x, const vg_solve_opts& o, vg_solve_
         int it = 0;
         const double gain = finish_correction(out, it);
         total += it;
-        // r.z not positive: the cycle, whose coarse levels have estimated weights, is not definite on these values. The
-        // hierarchy is made safe, and a correction that did harm is taken back.
-        if (rel > o.tol && use_amg && !amg_safe_ && !(out.sc.rz > 0 && out.sc.rz0 > 0)) {
-            make_amg_safe();
+        // A correction that did harm is taken back. Where r.z was not positive, the cycle, whose coarse levels have
+        // estimated weights, is not definite on these values, and the hierarchy is made safe; else the loop went on below
+        // its rounding level, and FP64 loops of six digits each follow.
+        const bool harm = !(rel <= 2.0 * before), indefinite = use_amg && !amg_safe_ && !(out.sc.rz > 0 && out.sc.rz0 > 0);
+        if (rel > o.tol && (harm || indefinite)) {
             if (!(rel < before)) {
                 if (direct)
                     VG_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * N, s));
@@ -994,6 +996,14 @@ void Solver::solve(const double* b, double* x, const vg_solve_opts& o, vg_solve_
                 true_residual();
                 rel = read();
                 n_launch += 1;
+            }
+            if (indefinite) {
+                make_amg_safe();
+            } else if (careful) {
+                ++outer;
+                break;
+            } else {
+                fp64 = careful = true;
             }
             continue;
         }

@@ -84,7 +84,7 @@ __device__ void grid_reduce(double (&v)[NV], double* partials, unsigned* counter
 }
 
 __device__ __forceinline__ double cg_alpha(const Scalars* sc) {
-    return sc->pq > 0 && isfinite(sc->pq) ? sc->rz / sc->pq : 0.0;
+    return sc->pq > CG_BREAK * sc->rz && isfinite(sc->pq) ? sc->rz / sc->pq : 0.0;
 }
 
 // an entry's share of r.D^{-1} r and of |r|^2 + |D^{-1} r|^2 (the jump's effect on the pressure and on the flux rows);
@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(VEC_THREADS) k_cg_finish(CgVecs<T> v, int firs
                 sc->best = rz;
                 sc->best_it = flags[2];
             }
-            if (!ok || !(sc->pq > 0) || flags[2] - sc->best_it >= CG_STALL || (rz <= sc->tol2 * sc->rz0 && sc->raw <= sc->raw2) || rz <= sc->floor2 * sc->rz0)
+            if (!ok || !(sc->pq > CG_BREAK * sc->rz) || cg_spent(rz, sc->best, flags[2] - sc->best_it, sc->rz0) || (rz <= sc->tol2 * sc->rz0 && sc->raw <= sc->raw2) || rz <= sc->floor2 * sc->rz0)
                 flags[0] = 1;
         }
         sc->rz = rz;

@@ -19,8 +19,17 @@ struct Scalars {
 // flags[0] = stop (converged or breakdown), flags[2] = iterations
 constexpr int NFLAGS = 4;
 
-// an iteration count without a new smallest r.z after which the loop gives up (rounding level reached)
-constexpr int CG_STALL = 1000;
+// What ends a loop that has not met its test: r.z far above the smallest one so far, or no new smallest one for long. A
+// loop that has gained ten digits is at its rounding level and is given neither. With the flux given the constants are in
+// the kernel of S; what rounding has put of them into r then grows from step to step and takes the digits of x with it, so
+// that such a loop has to end at once (33 cells, 1e4 in permeability between them, tolerance 1e-12: residual 3e16 after
+// 1,136 iterations; now 5e-14 after 33). Solves of degree 4 take 400 to 600 iterations either way.
+__host__ __device__ inline bool cg_spent(double rz, double best, int since, double rz0) {
+    const bool deep = best <= 1e-20 * rz0;
+    return rz > (deep ? 1e2 : 1e8) * best || since >= (deep ? 100 : 1000);
+}
+// A step of more than 1 / CG_BREAK along p is none: p is a constant then and p.q rounding.
+constexpr double CG_BREAK = 1e-10;
 
 constexpr int VEC_BLOCKS = 148 * 4;  // grid of the vector kernels (fixed: deterministic reductions)
 constexpr int VEC_THREADS = 256;

@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(ST, 1) k_small_cg(SmallCg<T> a) {
                 best = now;
                 best_it = its;
             }
-            stop = !fine || !(pq > 0) || its - best_it >= CG_STALL ||
+            stop = !fine || !(pq > CG_BREAK * rz) || cg_spent(now, best, its - best_it, rz0) ||
                    (now <= a.stop.tol * a.stop.tol * rz0 && raw <= raw2) ||
                    now <= a.stop.floor * a.stop.floor * rz0 || its >= a.maxit;
         }
@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(ST, 1) k_small_cg(SmallCg<T> a) {
         double t[1];
         get_sums<1>(part, t);
         pq = t[0];
-        const T alpha = T(pq > 0 && isfinite(pq) ? rz / pq : 0.0);
+        const T alpha = T(pq > CG_BREAK * rz && isfinite(pq) ? rz / pq : 0.0);
         if (coarse) {
             put_cell(warp, sr - alpha * sq);
             for (int k = warp + SW; k < np; k += SW) {
