@@ -38,15 +38,15 @@ namespace vg {
 namespace {
 
 // Largest mesh of degree 0 whose loop runs as one launch (vg_small.cu), and at degree k a (k + 1)th of it. What ends the
-// gain is that a CTA's constants no longer fit its shared memory and that its pieces follow one another. From degree 3 on
-// the condensed blocks alone decide, which grow with (k + 1)^2 and come in whole pieces: a CTA holds SMALL_BLOCKS bytes of
-// them at most (one piece in FP64, two or three in FP32). One launch against one kernel per phase, ms per solve to 1e-10
-// (disk; FP64, then mixed):
-//   k = 0   30,000 0.67 : 0.88, 0.67 : 1.01    64,000 1.15 : 1.00, 1.15 : 1.08    90,000 1.63 : 1.20, 1.62 : 1.24
-//   k = 1   16,000 1.36 : 1.83, 1.10 : 1.51    32,000 2.04 : 2.19, 1.90 : 2.28    45,000 2.70 : 2.36, 2.38 : 2.49
-//   k = 2   10,000 6.2 : 8.2, 5.7 : 7.6        21,000 12.5 : 13.1, 8.6 : 9.1      30,000 12.7 : 12.9, 9.5 : 9.2
-//   k = 3    4,000 15.8 : 29.6, 16.6 : 23.2     8,000 34.1 : 30.5, 18.9 : 25.4    16,000 45.4 : 45.6, 25.6 : 28.6
-//   k = 4    4,000 54 : 105, 43 : 67            8,000 130 : 105, 58 : 78          12,800 162 : 136, 127 : 86
+// gain is that a CTA's constants no longer fit its shared memory and that its pieces follow one another. At degree 4 the
+// condensed blocks alone decide, which grow with (k + 1)^2 and come in whole pieces: a CTA holds SMALL_BLOCKS bytes of
+// them at most (one piece in FP64, two in FP32). One launch against one kernel per phase, ms per solve to 1e-10 (disk;
+// FP64, then mixed; the graph's vary by a tenth and more with the handle's place in memory at degrees 2 to 4):
+//   k = 0   30,000 0.67 : 0.91, 0.67 : 0.96    60,000 0.95 : 1.03, 0.95 : 1.14    64,000 1.15 : 1.02, 1.15 : 1.07
+//   k = 1   16,000 1.33 : 1.90, 1.07 : 1.51    32,000 2.04 : 2.16, 1.89 : 2.28    45,000 2.70 : 2.33, 2.37 : 2.49
+//   k = 2   12,000 6.8 : 9.1, 6.2 : 8.1        21,000 12.1 : 14.4, 8.5 : 9.1      30,000 12.5 : 10.7, 9.5 : 9.2
+//   k = 3    4,000 15.7 : 28.2, 15.9 : 22.2     8,000 36 : 31, 20 : 26            16,000 46 : 60, 26 : 30
+//   k = 4    4,000 55 : 105, 43 : 64            8,000 134 : 110, 59 : 73          12,800 157 : 142, 126 : 84
 constexpr long long SMALL_BLOCKS = 120 << 10;
 constexpr int SMALL_CELLS = 64000;
 constexpr int HT = 256;
@@ -467,7 +467,7 @@ void Solver::plan_hybrid() {
     const long long per_cta = (long long)(pieces_.size() + sm_count_ - 1) / sm_count_;
     auto small = [&](size_t elem) {
         return m.nc <= SMALL_CELLS / (k + 1) &&
-               (k < 3 || s_total_ / (long long)pieces_.size() * per_cta * (long long)elem <= SMALL_BLOCKS);
+               (k < 4 || s_total_ / (long long)pieces_.size() * per_cta * (long long)elem <= SMALL_BLOCKS);
     };
     small_ctas_[0] = small(sizeof(double)) ? small_cg_ctas<double>(k, int(pieces_.size()), (long long)(k + 1) * m.ne, m.nc) : 0;
     small_ctas_[1] = k >= 1 && small(sizeof(float)) ? small_cg_ctas<float>(k, int(pieces_.size()), (long long)(k + 1) * m.ne, m.nc) : 0;
