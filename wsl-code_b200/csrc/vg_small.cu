@@ -587,7 +587,6 @@ int small_cg_ctas(int k, int npieces, long long n, int cells) {
 
 template <typename T>
 void launch_small_cg(const SmallCg<T>& a, int ctas, cudaStream_t s) {
-    VG_CUDA(cudaMemsetAsync(a.barrier, 0, sizeof(unsigned), s));
     SmallCg<T> args = a;
     args.smem = SMALL_SMEM;
     void* p[] = {&args};
