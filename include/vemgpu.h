@@ -144,12 +144,17 @@ int vg_sizes(const vg_handle* h, long long out[9]);
 int vg_set_problem(vg_handle* h, int problem, int bc);
 
 /* Per-cell log permeability theta (K_E = exp(theta_E) I): host (on_device = 0) or device pointer.
+ * After vg_build the operator and what vg_solve keeps get the new values in this call, on the structure they have (the
+ * aggregates are those of the field the handle was built with: one built with a rough field itself takes fewer iterations).
  * New in this library; the reference hard-codes K = I (vem/CurvedVEM_Darcy_gpu/src/equation_gpu.cu:63-68). */
 int vg_set_log_permeability(vg_handle* h, const double* theta, int on_device);
 
 /* FP64 setup on the device: geometry, projector and local operators (HdivGpu::build_basis,
  * hdiv_gpu.cu:172-192, + MixedGpu::update, equation_gpu.cu:547-577), right-hand side and boundary
- * data (MixedGpu::make_rhs, equation_gpu.cu:611-625) and the preconditioner. */
+ * data (MixedGpu::make_rhs, equation_gpu.cu:611-625) and, with the pressure condition, what vg_solve keeps: the
+ * condensed cells, the edge system and its multigrid. With the flux condition the first vg_solve after vg_build (or after
+ * vg_set_problem and vg_build) makes these, outside vg_solve_info.seconds, since a Maxwell-Stefan handle never needs them
+ * (4,096 quadrilaterals, degree 1: 4.4 ms of a first solve's 5.6). */
 int vg_build(vg_handle* h);
 
 /* ---- operator ----------------------------------------------------------------------------- */
@@ -229,7 +234,8 @@ int vg_cell_areas(vg_handle* h, double* areas);
  * diffusivities D12, D13, D23: backward Euler, one coupled saddle-point system per step with the
  * friction matrix frozen at x^n, no flux through the boundary (the handle must be built with
  * VG_BC_FLUX; its K = I operator is used whatever the permeability). State vector (device doubles):
- * [J1 (nf), J2 (nf), x1 (num_cells), x2 (num_cells)], x3 = 1 - x1 - x2. */
+ * [J1 (nf), J2 (nf), x1 (num_cells), x2 (num_cells)], x3 = 1 - x1 - x2. The call condenses the cells for the edge
+ * system (once per vg_build); the first vg_ms_step after it builds the species' multigrid on the host from its state. */
 int vg_ms_configure(vg_handle* h, double d12, double d13, double d23, double dt, long long* state_size);
 /* y = K(coeff_state) x for the Maxwell-Stefan system (FP64 or FP32 x, y; device). */
 int vg_ms_apply(vg_handle* h, const double* coeff_state, const void* x, void* y, int precision);

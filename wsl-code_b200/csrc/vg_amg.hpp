@@ -1,6 +1,7 @@
 // Smoothed-aggregation algebraic multigrid for a weighted graph Laplacian S on the cells: the coarse
-// part of the edge-pressure preconditioner (vg_hybrid.cu), and per species the pressure Schur block
-// (|E|/dt) I + W diag(F^{-1}) W^T of a Maxwell-Stefan step.
+// part of the edge-pressure preconditioner (vg_hybrid.cu); per species that of a Maxwell-Stefan step
+// (vg_ms.cu: conductances 1 / (sum over an edge's sides of 1 / (T_ii (B^{-1})_ss)), plus |E|/dt); and the
+// pressure rows of MINRES (vg_minres.cu: conductances 1 / A_ii).
 //
 // The reference preconditions with a PETSc ILU(0) on the CPU or, matrix-free, with the diagonal
 // |rate M| + sum W^2/d (vem/CurvedVEM_Darcy_gpu/src/krylov.cu:99-117, src/equation_gpu.cu:282-315),

@@ -478,7 +478,7 @@ void Solver::plan_hybrid() {
     d_eS32_.resize(strided ? size_t(s_total_) : 0);
     const size_t n = size_t(k + 1) * m.ne;
     d_edinv64_.resize(n);
-    d_eh_.resize(n + 1);  // + the barrier word of the single-launch loop, cleared with it
+    d_eh_.resize(n + 1);  // + the barrier word of the single-launch loop, which correct() clears with it
     d_erelax64_.resize(n);
     d_erelax32_.resize(n);
     d_econd_.resize(m.ne);
@@ -791,15 +791,15 @@ void Solver::build_graph(int p) {
     VG_CUDA(cudaGraphInstantiate(&gexec_[p], graph_[p], 0));
 }
 
-// conjugate gradients for the correction d of the residual r (symmetric form, internal order): condensed
-// right-hand side, loop, back substitution (d's flux rows zero on entry). Returns the loop's gain in the preconditioned
-// norm. The caller reads the outcome with finish_correction once more work is queued behind it.
 template <typename T>
 bool Solver::takes_one_launch() {
     AmgView<T> v;
     return small_ctas_[sizeof(T) == 4 ? 1 : 0] > 0 && (!use_amg || amg_.view_levels<T>(v));
 }
 
+// conjugate gradients for the correction d of the residual r (symmetric form, internal order): condensed
+// right-hand side, loop, back substitution (d's flux rows zero on entry). The caller reads the outcome with
+// finish_correction once more work is queued behind it.
 template <typename T>
 void Solver::correct(const double* r, double* d, const CgStop& stop, int maxit, int check_every, cudaStream_t s) {
     Scalars* sc = scalars();

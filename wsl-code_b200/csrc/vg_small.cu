@@ -1,8 +1,8 @@
 // Conjugate gradients on the edge pressures of a small mesh as one cooperative launch.
 //
-// The loop of vg_krylov.cu runs 5 dependent kernels an iteration plus 2 per multigrid level. Up to some ten
-// thousand cells each of them has work for a microsecond or two and costs 5 to 6 of launch, drain and grid
-// reduction (1,000 cells FP64: 33 us an iteration). Here the grid stays resident, one CTA per SM, and the phases
+// The loop of vg_krylov.cu runs 5 dependent kernels an iteration plus 2 per multigrid level. On a small mesh (the
+// line is in vg_hybrid.cu: 64,000 cells at degree 0) each of them has work for a microsecond or two and costs 5 to 6
+// of launch, drain and grid reduction (1,000 cells FP64: 33 us an iteration). Here the grid stays resident, one CTA per SM, and the phases
 // of an iteration are separated by grid barriers:
 //   apply      q += S p, p.q                                  (one lane per cell, red.global.add into zeroed q)
 //   update     x += alpha p, r' = r - alpha q, sums; rc = Pi^T (r - alpha q)

@@ -215,7 +215,7 @@ private:
         static int dot_blocks(long long n, long long chunk) { return int((n + chunk - 1) / chunk); }
         cudaGraph_t graph[2] = {nullptr, nullptr};  // captured Arnoldi loops (FP64, FP32)
         cudaGraphExec_t gexec[2] = {nullptr, nullptr};
-        // per-species multigrid of the pressure Schur block, built from the first state stepped
+        // per-species multigrid of the cells' graph, built from the first state stepped
         // after vg_ms_configure and kept for the following steps
         Amg amg[2];
         bool amg_ready = false;
