@@ -185,15 +185,16 @@ int vg_apply(vg_handle* h, const void* x, void* y, int precision, int constraine
         cudaStream_t st = static_cast<cudaStream_t>(stream);
         const bool internal = (precision & VG_ORDER_INTERNAL) != 0;
         precision &= ~VG_ORDER_INTERNAL;
+        // the flux rows are summed into; every pressure row and the multiplier's is stored by its owner
         if (precision == VG_FP64) {
-            VG_CUDA(cudaMemsetAsync(y, 0, sizeof(double) * s.N, st));
+            VG_CUDA(cudaMemsetAsync(y, 0, sizeof(double) * s.nf, st));
             if (internal)
                 s.apply_int<double>(static_cast<const double*>(x), static_cast<double*>(y), constrained != 0, 1.0, st,
                                     nullptr);
             else
                 s.apply64(static_cast<const double*>(x), static_cast<double*>(y), constrained != 0, 1.0, st);
         } else if (precision == VG_FP32) {
-            VG_CUDA(cudaMemsetAsync(y, 0, sizeof(float) * s.N, st));
+            VG_CUDA(cudaMemsetAsync(y, 0, sizeof(float) * s.nf, st));
             if (internal)
                 s.apply_int<float>(static_cast<const float*>(x), static_cast<float*>(y), constrained != 0, 1.0f, st,
                                    nullptr);
