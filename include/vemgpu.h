@@ -14,7 +14,9 @@
  *     when the boundary condition is VG_BC_FLUX (vem/CurvedVEM_Darcy/solver/DarcySolver.cpp:182-227);
  *   - all functions return 0 on success or a VG_E* code; vg_last_error() describes the failure.
  *     No C++ exception crosses this boundary (vem/CurvedVEM_Darcy_gpu/src/krylov.cu:8-36).
- *   - a handle is not re-entrant: one host thread at a time (vem/CurvedVEM_Darcy_gpu/include/petsc_gpu.h:5).
+ *   - a handle is not re-entrant: one host thread at a time (vem/CurvedVEM_Darcy_gpu/include/petsc_gpu.h:5). Nor may
+ *     calls on other handles of the process run beside a handle's first vg_solve, vg_adjoint_grad or vg_ms_step of a mode,
+ *     which captures its loop: a device-wide wait in another thread breaks the capture.
  */
 #ifndef VEMGPU_H
 #define VEMGPU_H
